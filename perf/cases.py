@@ -85,12 +85,6 @@ def draw(rng):
             return c
 
 
-def _even(rng, lo, hi):
-    """A texture size. Even: a one-channel 8-bit map of odd size once left the
-    maps after it at odd addresses, a fault of the GPU in code of that time."""
-    return 2 * _log(rng, lo / 2, hi / 2)
-
-
 def _draw(rng):
     kind = rng.choice(["cornell", "cornell", "field", "field", "room", "stress", "batch", "photon", "load", "rays"])
     w = _log(rng, 65, 1920)
@@ -103,16 +97,16 @@ def _draw(rng):
         return dict(frame, spheres=_log(rng, 30, 800), depth=rng.randint(6, 16), mis=rng.random() < 0.8,
                     lens=rng.random() < 0.6, dispersion=rng.random() < 0.3, aovs=aovs)
     if kind == "room":
-        return dict(frame, depth=rng.randint(4, 16), tex=_even(rng, 34, 700), mis=rng.random() < 0.8, aovs=aovs)
+        return dict(frame, depth=rng.randint(4, 16), tex=_log(rng, 33, 700), mis=rng.random() < 0.8, aovs=aovs)
     if kind == "stress":
-        return dict(frame, spheres=_log(rng, 40, 400), cuboids=_log(rng, 20, 500), tex=_even(rng, 66, 512),
+        return dict(frame, spheres=_log(rng, 40, 400), cuboids=_log(rng, 20, 500), tex=_log(rng, 65, 512),
                     depth=rng.randint(12, 32), aovs=aovs)
     if kind == "batch":
         return {"kind": kind, "jobs": rng.randint(2, 12), "mix": rng.randint(0, 1 << 20), "spp": _log(rng, 4, 32)}
     if kind == "photon":
         w = _log(rng, 97, 640)
         return {"kind": kind, "width": w, "height": max(64, int(w * rng.uniform(0.6, 1.0))),
-                "iterations": rng.randint(1, 4), "depth": rng.randint(4, 12), "tex": _even(rng, 34, 512)}
+                "iterations": rng.randint(1, 4), "depth": rng.randint(4, 12), "tex": _log(rng, 33, 512)}
     if kind == "load":
         return {"kind": kind, "spheres": _log(rng, 20, 400), "width": w // 4 + 16, "height": h // 4 + 16}
     return {"kind": kind, "spheres": _log(rng, 20, 200), "rays": _log(rng, 1000, 1500000)}
