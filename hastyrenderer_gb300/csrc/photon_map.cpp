@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -109,6 +110,23 @@ float close_non_negative(const float* img, int W, int H, int i, int j) {
   return 1e-3f;
 }
 
+// fn(0) .. fn(n - 1), each once, on up to n threads, the calling one among them.
+// It takes over what is left where the system gives no further thread, and
+// joins the ones it started. fn does not throw.
+template <class Fn>
+void run_parts(size_t n, Fn fn) {
+  std::atomic<size_t> next{0};
+  auto work = [&] { for (size_t k; (k = next.fetch_add(1)) < n;) fn(k); };
+  std::vector<std::thread> th;
+  th.reserve(n);
+  try {
+    while (th.size() + 1 < n) th.emplace_back(work);
+  } catch (const std::system_error&) {
+  }
+  work();
+  for (std::thread& t : th) t.join();
+}
+
 // The cost of four cell sizes: float sums over the radii in the order given.
 typedef float f4 __attribute__((vector_size(16)));
 f4 cell_costs(const float* radii, size_t n, f4 c) {
@@ -152,14 +170,8 @@ float cell_size_for(const float* radii, size_t n) {
     for (int k = 0; k < 2; ++k) { cd[at][k] = c[k]; cd[at + 1][k] = c[2 + k]; }
     n_down[at] = n_down[at + 1] = 2;
   };
-  if (n >= (size_t(1) << 15)) {
-    std::thread a([&] { first_down(0); }), b([&] { first_down(2); });
-    more_up();
-    a.join();
-    b.join();
-  } else {
-    more_up();
-  }
+  if (n >= (size_t(1) << 15)) run_parts(3, [&](size_t k) { if (k == 0) more_up(); else first_down(2 * int(k) - 2); });
+  else more_up();
   float best = cu[0];
   int at = 0;
   for (int k = 1; k <= 10; ++k) {
@@ -189,10 +201,42 @@ template <class Fn>
 void parallel_ranges(size_t n, size_t least, Fn fn) {
   const size_t hw = std::max(1u, std::thread::hardware_concurrency());
   const size_t nt = std::max<size_t>(1, std::min({n / std::max<size_t>(least, 1), hw, size_t(8)}));
-  std::vector<std::thread> th;
-  for (size_t k = 1; k < nt; ++k) th.emplace_back([&, k] { fn(n * k / nt, n * (k + 1) / nt); });
-  fn(0, n / nt);
-  for (std::thread& t : th) t.join();
+  run_parts(nt, [&](size_t k) { fn(n * k / nt, n * (k + 1) / nt); });
+}
+
+// d: the pixels' distances (computeRadiusPixelFootPrint, negative: none), row
+// by row, replaced by the footprint radii x 10. The angle's arctangents belong
+// to a column or a row; what is left per pixel is one tangent, on several
+// threads (640x480: 9.2 ms -> 1.1 ms in all).
+void footprint_radii(float* d, uint32_t W, uint32_t H, const std::vector<float>& ax, const std::vector<float>& ay) {
+  std::atomic<bool> holes{false};
+  parallel_ranges(H, (size_t(1) << 14) / W + 1, [&](size_t y0, size_t y1) {
+    bool hole = false;
+    for (size_t y = y0; y < y1; y++)
+      for (size_t x = 0; x < W; x++) {
+        const size_t p = y * W + x;
+        float fp = -1.0f;                       // computeRadiusPixelFootPrint's default
+        if (d[p] >= 0.0f) {
+          float angle = 0.5f * ax[x] + 0.5f * ay[y];
+          fp = 0.5f * d[p] * std::tan(angle);
+        }
+        d[p] = 10.0f * fp;
+        hole = hole || d[p] < 0.0f;
+      }
+    if (hole) holes = true;
+  });
+  if (holes)                                     // one after the other: a filled pixel counts for the next ones
+    for (uint32_t y = 0; y < H; y++)
+      for (uint32_t x = 0; x < W; x++)
+        if (d[size_t(y) * W + x] < 0.0f) d[size_t(y) * W + x] = close_non_negative(d, int(W), int(H), int(x), int(y));
+}
+
+// The angle terms of every column and row; q = tan(fov / 2).
+void footprint_angles(float q, uint32_t W, uint32_t H, std::vector<float>& ax, std::vector<float>& ay) {
+  ax.resize(W);
+  ay.resize(H);
+  for (uint32_t x = 0; x < W; x++) ax[x] = axis_angle(q, float(x) + 0.5f, float(W), float(W));
+  for (uint32_t y = 0; y < H; y++) ay[y] = axis_angle(q, float(y) + 0.5f, float(H), float(W));
 }
 
 template <class T>
@@ -243,8 +287,6 @@ void read_radii(hasty_job& j, PmDev& pm) {
 
 // Pixel statistics cleared and the radius image set up (renderPhotonThread,
 // PhotonMapping.cpp:828-833: footprint radii x 10 with a surface light, else 1).
-// The angle's arctangents belong to a column or a row; what is left per pixel
-// is one tangent, on several threads (640x480: 9.2 ms -> 1.1 ms in all).
 void pm_init(hasty_job& j, PmDev& pm) {
   const uint32_t W = pm.W, H = pm.H;
   const size_t n = size_t(W) * H;
@@ -262,31 +304,10 @@ void pm_init(hasty_job& j, PmDev& pm) {
     launch_pm_footprint(j.sd, j.seed, pm.px.radii, j.stream);
     ck(cudaGetLastError(), "footprint launch");
     ck(cudaMemcpyAsync(d, pm.px.radii, n * sizeof(float), cudaMemcpyDeviceToHost, j.stream), "footprint");
-    const float q = j.sd.cam.q;
-    std::vector<float> ax(W), ay(H);
-    for (uint32_t x = 0; x < W; x++) ax[x] = axis_angle(q, float(x) + 0.5f, float(W), float(W));
-    for (uint32_t y = 0; y < H; y++) ay[y] = axis_angle(q, float(y) + 0.5f, float(H), float(W));
+    std::vector<float> ax, ay;
+    footprint_angles(j.sd.cam.q, W, H, ax, ay);
     ck(cudaStreamSynchronize(j.stream), "footprint");
-    std::atomic<bool> holes{false};
-    parallel_ranges(H, (size_t(1) << 14) / W + 1, [&](size_t y0, size_t y1) {
-      bool hole = false;
-      for (size_t y = y0; y < y1; y++)
-        for (size_t x = 0; x < W; x++) {
-          const size_t p = y * W + x;
-          float fp = -1.0f;                     // computeRadiusPixelFootPrint's default
-          if (d[p] >= 0.0f) {
-            float angle = 0.5f * ax[x] + 0.5f * ay[y];
-            fp = 0.5f * d[p] * std::tan(angle);
-          }
-          d[p] = 10.0f * fp;
-          hole = hole || d[p] < 0.0f;
-        }
-      if (hole) holes = true;
-    });
-    if (holes)                                   // one after the other: a filled pixel counts for the next ones
-      for (uint32_t y = 0; y < H; y++)
-        for (uint32_t x = 0; x < W; x++)
-          if (d[size_t(y) * W + x] < 0.0f) d[size_t(y) * W + x] = close_non_negative(d, int(W), int(H), int(x), int(y));
+    footprint_radii(d, W, H, ax, ay);
     ck(cudaMemcpyAsync(pm.px.radii, d, n * sizeof(float), cudaMemcpyHostToDevice, j.stream), "radii");
   } else {
     launch_pm_fill(pm.px.radii, n, 1.0f, j.stream);
@@ -558,6 +579,17 @@ int hasty_debug_pm_table(hasty_job* job, int64_t max_cells) {
   return guarded([&] {
     pm_job(job);
     pm_state(*job).max_table = std::min(max_cells, kPmDenseCells);
+    return HASTY_OK;
+  });
+}
+
+int hasty_debug_pm_host(float* dist, size_t w, size_t h, float q, float* cell) {
+  return guarded([&] {
+    if (!dist || !cell || w == 0 || h == 0 || w > size_t(INT32_MAX) / h) throw ApiError{HASTY_ERR_ARG, "bad argument"};
+    std::vector<float> ax, ay;
+    footprint_angles(q, uint32_t(w), uint32_t(h), ax, ay);
+    footprint_radii(dist, uint32_t(w), uint32_t(h), ax, ay);
+    *cell = cell_size_for(dist, w * h);
     return HASTY_OK;
   });
 }

@@ -211,6 +211,11 @@ int hasty_debug_pm_map(hasty_job* job, float* xyz, uint32_t* emission, uint32_t*
 /* Test hook: the gather looks cells up in a table of all cells of the map's
  * bounds only up to max_cells of them (0: always searches the cell list). */
 int hasty_debug_pm_table(hasty_job* job, int64_t max_cells);
+/* Test hook (no device needed): the host's part of the photon mapper's set-up
+ * and of an iteration. dist: w x h distances (negative: none), replaced by the
+ * footprint radii of a camera with q = tan(fov / 2); cell: the hash-cell size
+ * for these radii, taken in the order they are stored in. */
+int hasty_debug_pm_host(float* dist, size_t w, size_t h, float q, float* cell);
 
 /* ---- Batching: many jobs in one multi-job wavefront ----------------------
  * Two modes.
