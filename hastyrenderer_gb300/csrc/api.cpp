@@ -473,11 +473,14 @@ void ray_list(hasty_job& j, int k, size_t rays) {
   if (rays <= j.ray_cap[k]) return;
   const size_t cap = (rays + 63) / 64 * 64;
   hasty::RayLists& l = j.ray_lists[k];
+  constexpr size_t kRayBytes = 10 * sizeof(float);
   if (l.rays) cudaFree(l.rays);
   l = {};
+  j.ray_bytes -= int64_t(j.ray_cap[k] * kRayBytes);
   j.ray_cap[k] = 0;
   float* p = nullptr;
-  ck(cudaMalloc(&p, cap * 10 * sizeof(float)), "cudaMalloc rays");
+  ck(cudaMalloc(&p, cap * kRayBytes), "cudaMalloc rays");
+  j.ray_bytes += int64_t(cap * kRayBytes);
   l = {p, reinterpret_cast<int32_t*>(p + 6 * cap), p + 7 * cap, p + 8 * cap, p + 9 * cap};
   j.ray_cap[k] = cap;
 }
@@ -628,7 +631,7 @@ int hasty_job_info_get(hasty_job* job, hasty_job_info* out) {
     out->n_shapes = int32_t(h.n_shapes); out->n_materials = int32_t(h.mats.size());
     out->env_is_texture = h.env_texture ? 1 : 0; out->exposure = h.cam.exposure;
     out->samples_done = job->samples_done; out->bvh_depth = job->bvh_depth; out->bvh_build_ms = job->bvh_ms;
-    out->device_bytes = job->bytes;
+    out->device_bytes = job->bytes + job->ray_bytes;
     out->bvh_tree_ms = job->bvh_tree_ms;
     out->parse_ms = job->parse_ms;
     out->upload_ms = job->upload_ms;
@@ -969,6 +972,7 @@ int hasty_debug_intersect(hasty_job* job, const float* rays, size_t n, int32_t* 
     // while the one before is traced. (1M rays: device allocations 0.25 ms and
     // an interleaved hit array taken apart on the host 2.1 ms, around 0.38 ms
     // of copies and tracing.)
+    ck(cudaSetDevice(job->ctx->device), "cudaSetDevice");   // the lists, stream and event stay with the job
     std::lock_guard<std::mutex> lock(job->ray_mutex);
     const size_t chunk = std::min(n, hasty_job::kRayChunk);
     const int lists = n > chunk ? 2 : 1;

@@ -141,6 +141,7 @@ struct hasty_job {
   std::mutex ray_mutex;
   hasty::RayLists ray_lists[2] = {};
   size_t ray_cap[2] = {0, 0};
+  std::atomic<int64_t> ray_bytes{0};  // of both lists (not in `bytes`: such a call may run beside ones that allocate)
   cudaStream_t ray_stream = nullptr;
   cudaEvent_t ray_ready = nullptr;
   bool stage_timing = false;
