@@ -173,9 +173,11 @@ void prepare_scene(hasty_job& j) {
   j.prep = std::move(p);
 }
 
-// A job's scene arrays share one device block (and its mesh arrays, which
-// only live until the shading records are made, another), carved in the order
-// of use: a load makes two allocations instead of one per array.
+// A job's scene arrays share one device block, carved in the order of use. The
+// mesh arrays, which only live until the shading records are made of them, use
+// the place of the arrays that come after the records, so that a load needs no
+// more device memory than the scene keeps. They go there in slices where they
+// are larger than those arrays (spheres: 98 bytes per triangle against 83).
 constexpr size_t kArenaAlign = 256;
 struct Arena {
   uint8_t* base = nullptr;     // null: only counts
@@ -196,22 +198,56 @@ struct Arena {
   }
 };
 
+constexpr int64_t kMeshSlice = 4096;     // triangles at a time, at least
+
+// What all slices of the triangles refer to, and slice [first, first + n).
 MeshDev put_mesh(const HostScene& h, Arena& a, cudaStream_t st) {
   MeshDev m{};
-  m.n_tris = int32_t(h.n_tris());
-  m.tri_pos = a.put(h.tri_pos, st);
-  m.tri_attr = a.put(h.tri_attr, st);
   m.normals = a.put(h.normals, st);
   m.texcoords = a.put(h.texcoords, st);
   m.n_texcoords = int64_t(h.texcoords.size());
   return m;
 }
+void put_slice(const HostScene& h, int64_t first, int64_t n, MeshDev& m, Arena& a, cudaStream_t st) {
+  m.n_tris = int32_t(n);
+  float* pos = a.take<float>(9 * size_t(n));
+  TriAttr* attr = a.take<TriAttr>(size_t(n));
+  m.tri_pos = pos;
+  m.tri_attr = attr;
+  if (!a.base || n == 0) return;
+  ck(cudaMemcpyAsync(pos, &h.tri_pos[9 * size_t(first)], 9 * size_t(n) * sizeof(float), cudaMemcpyHostToDevice, st), "upload");
+  ck(cudaMemcpyAsync(attr, &h.tri_attr[size_t(first)], size_t(n) * sizeof(TriAttr), cudaMemcpyHostToDevice, st), "upload");
+}
 
-// The scene's arrays and tables (mesh: null when only counting).
-void put_scene(const HostScene& h, const hasty_job::Prepared& p, const MeshDev* mesh, Arena& a, SceneDev& s, cudaStream_t st) {
+// The shading records of all triangles, by slices through `room` bytes at `at`.
+void put_records(const HostScene& h, float4* rec, uint8_t* at, size_t room, cudaStream_t st) {
+  Arena a;
+  a.base = at;
+  MeshDev mesh = put_mesh(h, a, st);
+  const size_t used = a.used;
+  const int64_t n = int64_t(h.n_tris());
+  constexpr size_t kTriBytes = 9 * sizeof(float) + sizeof(TriAttr);
+  const int64_t fit = room > used + 2 * kArenaAlign ? int64_t((room - used - 2 * kArenaAlign) / kTriBytes) : 0;
+  const int64_t slice = std::max(kMeshSlice, fit);
+  for (int64_t first = 0; first < n; first += slice) {
+    a.used = used;
+    put_slice(h, first, std::min(slice, n - first), mesh, a, st);
+    launch_tri_records(mesh, rec + kTriRecord * first, st);
+  }
+}
+// Room that put_records needs at least.
+size_t records_room(const HostScene& h) {
+  Arena a;
+  MeshDev m = put_mesh(h, a, nullptr);
+  put_slice(h, 0, std::min<int64_t>(kMeshSlice, int64_t(h.n_tris())), m, a, nullptr);
+  return a.used;
+}
+
+// The scene's arrays and tables; total: the block's bytes, 0 when only counting.
+void put_scene(const HostScene& h, const hasty_job::Prepared& p, size_t total, Arena& a, SceneDev& s, cudaStream_t st) {
   float4* rec = a.take<float4>(size_t(kTriRecord) * h.n_tris());
-  if (mesh) launch_tri_records(*mesh, rec, st);
   s.tri_rec = rec;
+  if (a.base) put_records(h, rec, a.base + a.used, total - a.used, st);
   s.nodes = reinterpret_cast<const float4*>(a.put(p.bvh.nodes, st));
   s.isect_tris = reinterpret_cast<const float4*>(a.put(p.bvh.tris, st));
   s.mats = a.put(h.mats, st);
@@ -233,16 +269,14 @@ void put_scene(const HostScene& h, const hasty_job::Prepared& p, const MeshDev* 
   e.cdf = reinterpret_cast<const uint64_t*>(env_cdf);
 }
 
-size_t mesh_bytes(const HostScene& h) { Arena a; put_mesh(h, a, nullptr); return a.used; }
+// Device bytes of a prepared scene: what upload_scene allocates and keeps.
 size_t scene_bytes(const HostScene& h, const hasty_job::Prepared& p) {
-  Arena a;
+  Arena rec, all;
+  rec.take<float4>(size_t(kTriRecord) * h.n_tris());
   SceneDev s{};
-  put_scene(h, p, nullptr, a, s, nullptr);
-  return a.used;
+  put_scene(h, p, 0, all, s, nullptr);
+  return std::max(all.used, rec.used + records_room(h));
 }
-
-// Device bytes upload_scene allocates for a prepared job (its peak).
-int64_t upload_bytes(const hasty_job& j) { return int64_t(mesh_bytes(j.host) + scene_bytes(j.host, *j.prep)); }
 
 void upload_scene(hasty_job& j) {
   prepare_scene(j);
@@ -251,12 +285,11 @@ void upload_scene(hasty_job& j) {
   SceneDev& s = j.sd;
   hasty_job::Prepared& p = *j.prep;
   j.bvh_depth = p.bvh.depth; j.bvh_ms = p.bvh.build_ms; j.bvh_tree_ms = p.bvh.tree_ms;
-  Arena scene, tmp;
-  scene.base = j.alloc<uint8_t>(scene_bytes(h, p));
-  tmp.base = j.alloc<uint8_t>(mesh_bytes(h));
-  const MeshDev mesh = put_mesh(h, tmp, j.stream);
-  put_scene(h, p, &mesh, scene, s, j.stream);
-  s.n_tris = mesh.n_tris;
+  Arena scene;
+  const size_t total = scene_bytes(h, p);
+  scene.base = j.alloc<uint8_t>(total);
+  put_scene(h, p, total, scene, s, j.stream);
+  s.n_tris = int32_t(h.n_tris());
   s.bvh_kind = p.binary ? 0 : 1;
   s.n_nodes = int32_t(p.bvh.nodes.size() / (p.binary ? 16 : kWideNodeWords));
   s.n_mats = int32_t(h.mats.size());
@@ -279,7 +312,6 @@ void upload_scene(hasty_job& j) {
   s.p_surface = !h.env_texture ? 1.0f : (!h.light_tris.empty() ? 0.5f : 0.0f);   // Scene.cpp:545
   ck(cudaGetLastError(), "scene tables");
   ck(cudaStreamSynchronize(j.stream), "sync upload");   // the host arrays may be freed after this
-  j.release(tmp.base);
   j.upload_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - u0).count();
   j.prep.reset();
 }
@@ -527,7 +559,7 @@ std::unique_ptr<hasty_job> hasty::load_job(hasty_ctx* ctx, const std::string& pa
 
 int64_t hasty::prepare_job_upload(hasty_job& j) {
   prepare_scene(j);
-  return upload_bytes(j);
+  return int64_t(scene_bytes(j.host, *j.prep));
 }
 
 extern "C" {
