@@ -68,7 +68,6 @@ void hasty::carve_paths(PathsDev& p, int64_t cap, int n_stats, const std::functi
   p.rq[0] = static_cast<int32_t*>(A(2 * c * sizeof(int32_t)));
   p.rq[1] = static_cast<int32_t*>(A(2 * c * sizeof(int32_t)));
   p.counts = static_cast<uint32_t*>(A(kCountSlots * sizeof(uint32_t)));
-  p.sq = static_cast<int32_t*>(A(c * sizeof(int32_t)));
   p.out_color = static_cast<float4*>(A(c * sizeof(float4)));
   p.out_normal = static_cast<float4*>(A(c * sizeof(float4)));
   p.out_albedo = static_cast<float4*>(A(c * sizeof(float4)));
@@ -177,7 +176,7 @@ void prepare_scene(hasty_job& j) {
 // mesh arrays, which only live until the shading records are made of them, use
 // the place of the arrays that come after the records, so that a load needs no
 // more device memory than the scene keeps. They go there in slices where they
-// are larger than those arrays (spheres: 98 bytes per triangle against 83).
+// are larger than those arrays (spheres: 98 bytes per triangle, in 101).
 constexpr size_t kArenaAlign = 256;
 struct Arena {
   uint8_t* base = nullptr;     // null: only counts
@@ -392,8 +391,12 @@ int64_t hasty::path_kernel_max_triangles() {
   return v;
 }
 
+bool hasty::may_use_path_kernel(const hasty_ctx* ctx) {
+  return !(ctx->flags & HASTY_CTX_WAVEFRONT) && ((ctx->flags & HASTY_CTX_PATH_KERNEL) || path_kernel_max_triangles() > 0);
+}
+
 bool hasty::use_path_kernel(const hasty_ctx* ctx, const SceneDev& sc) {
-  if (sc.max_depth <= 0 || (ctx->flags & HASTY_CTX_WAVEFRONT)) return false;
+  if (sc.max_depth <= 0 || !may_use_path_kernel(ctx)) return false;
   return (ctx->flags & HASTY_CTX_PATH_KERNEL) || int64_t(sc.n_tris) <= path_kernel_max_triangles();
 }
 

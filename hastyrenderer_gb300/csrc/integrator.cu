@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(RT, 1024 / RT) k_resolve(const __grid_constant
       for (int c = 0; c < res.cls; ++c)
         for (int w = 0; w < kWarps; ++w) off += s_cnt[w][c];
       for (uint32_t w = 0; w < warp; ++w) off += s_cnt[w][res.cls];
-      P.sq[off] = s;
+      P.rq[q][off] = s;
     }
     const unsigned sb = __ballot_sync(kFull, res.shaded != 0);
     if (lane == 0 && sb) atomicAdd(&P.stats[ST_SHADED], (unsigned long long)__popc(sb));
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(ST, 1024 / ST) k_sample(const __grid_constant_
     const uint32_t i = first + threadIdx.x;
     if ((i & ~31u) < n_in) {
       bool valid = i < n_in;
-      int s = valid ? P.sq[i] : 0;
+      int s = valid ? P.rq[q][i] : 0;
       if (valid && !HASTY_IN_BOUNDS(s >= 0 && s < P.capacity, BB_QUEUE)) { valid = false; s = 0; }
       SampleRes res;
       res.keep = res.emitB = res.emitL = false;
@@ -1232,7 +1232,7 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_resolve_multi(PathsDev P
   uint32_t base = 0;
   if (lane == 0 && kb) base = atomicAdd(&P.counts[kSampleCount], uint32_t(__popc(kb)));
   base = __shfl_sync(kFull, base, 0);
-  if (res.sample) P.sq[base + __popc(kb & ((1u << lane) - 1u))] = s;
+  if (res.sample) P.rq[q][base + __popc(kb & ((1u << lane) - 1u))] = s;
   unsigned sb = __ballot_sync(kFull, res.shaded != 0);
   if (lane == 0 && sb) atomicAdd(&P.stats[ST_SHADED], (unsigned long long)__popc(sb));
 }
@@ -1242,7 +1242,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) k_sample_multi(PathsDev P, 
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if ((i & ~31u) >= n_in) return;
   const bool valid = i < n_in;
-  int s = valid ? P.sq[i] : 0;
+  int s = valid ? P.rq[m.ctl[0]][i] : 0;
   const uint4 meta = valid ? m.slot_meta[s] : make_uint4(0u, 0u, 0u, 0u);
   const int j = int(meta.x);
   SampleRes res;

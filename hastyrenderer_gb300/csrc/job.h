@@ -247,6 +247,8 @@ int lane_trace_blocks();
 // context says otherwise (HASTY_CTX_WAVEFRONT, HASTY_CTX_PATH_KERNEL).
 int64_t path_kernel_max_triangles();
 bool use_path_kernel(const hasty_ctx* ctx, const SceneDev& sc);
+// Whether it is for any scene of the context.
+bool may_use_path_kernel(const hasty_ctx* ctx);
 // Slot pool of the path kernel (path_slots() slots; its statistics are `stats`).
 void alloc_path_slots(PathsDev& p, const std::function<void*(size_t)>& alloc, unsigned long long* stats);
 }  // namespace hasty

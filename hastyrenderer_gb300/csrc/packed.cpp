@@ -22,8 +22,9 @@ void PackedLanes::init(hasty_ctx* c, int lanes, int64_t paths) {
   ck(cudaEventCreateWithFlags(&acc_ready, cudaEventDisableTiming), "event");
   // All lanes' buffers in one block: of 14.4 GB (two lanes of 16M paths), 36
   // allocations took 2.4 ms and their frees 11.1 ms; one takes 0.4 and 5.0.
-  // The path kernel's slot pools are part of it, so the lanes' footprint is
-  // fixed from the start.
+  // The path kernel's slot pools are part of it (40 MB per lane, in contexts
+  // whose scenes may use that kernel), so the lanes' footprint is fixed from
+  // the start.
   size_t used = 0;
   uint8_t* base = nullptr;
   const auto take = [&](size_t b) -> void* {
@@ -36,7 +37,7 @@ void PackedLanes::init(hasty_ctx* c, int lanes, int64_t paths) {
     stats = static_cast<unsigned long long*>(take(sizeof(unsigned long long) * ST_COUNT));
     for (int k = 0; k < n_lanes; ++k) {
       carve_paths(pd[k], lane_paths, ST_COUNT, take, stats);
-      alloc_path_slots(slots[k], take, stats);
+      if (may_use_path_kernel(ctx)) alloc_path_slots(slots[k], take, stats);
     }
   };
   carve();
@@ -50,7 +51,7 @@ void PackedLanes::init(hasty_ctx* c, int lanes, int64_t paths) {
     ck(cudaEventCreateWithFlags(&lane_done[k], cudaEventDisableTiming), "event");
     ck(cudaEventCreateWithFlags(&lane_free[k], cudaEventDisableTiming), "event");
     ck(cudaMemsetAsync(pd[k].counts, 0, sizeof(uint32_t) * kCountSlots, acc_stream), "memset counts");
-    ck(cudaMemsetAsync(slots[k].counts, 0, sizeof(uint32_t) * kCountSlots, acc_stream), "memset counts");
+    if (slots[k].counts) ck(cudaMemsetAsync(slots[k].counts, 0, sizeof(uint32_t) * kCountSlots, acc_stream), "memset counts");
   }
   wait_for(acc_stream);
 }

@@ -55,9 +55,9 @@ struct PathsDev {
   float4* ray;          // 2 per ray (2 rays per path): origin, w the path's chunk (bits); direction
   float4* hit;          // 1 per ray: t, u, v, triangle (-1 miss)
   int32_t* pq[2];       // path queues
-  int32_t* rq[2];       // ray queues (ray ids 2s, 2s+1)
+  int32_t* rq[2];       // ray queues (ray ids 2s, 2s+1); once traced, queue q is the sample queue of its
+                        // bounce (paths that continue past resolve)
   uint32_t* counts;     // [pq0, rq0, pq1, rq1, then kFetchCounter.. below]
-  int32_t* sq;          // sample queue (paths that continue past resolve)
   float4* out_color;    // per slot: final radiance of the sample
   float4* out_normal;
   float4* out_albedo;
