@@ -930,8 +930,7 @@ int path_grid_of(K kernel) {
   return std::max(1, sms) * std::max(1, per_sm);
 }
 int path_grid() {
-  static int g = 0;
-  if (!g) g = std::max(path_grid_of(k_paths<OneJob, 1, false>), path_grid_of(k_paths<ChunkTable, 1, false>));
+  static const int g = std::max(path_grid_of(k_paths<OneJob, 1, false>), path_grid_of(k_paths<ChunkTable, 1, false>));
   return g;
 }
 template <class Src>
