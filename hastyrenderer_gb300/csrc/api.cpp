@@ -463,18 +463,18 @@ void render_batch(hasty_job& j, int n_passes, int lane, bool more_batches) {
     // Stage timing measures the wavefront's stages, so it leaves the
     // finishing of small queues out.
     const bool finish = !(j.ctx->flags & HASTY_CTX_WAVEFRONT) && !j.stage_timing && j.sd.max_depth > 0;
-    const int64_t limit = finish ? finish_limit(simple_trace_bvh(j.sd)) : 0;
+    const FinishLimits limits = finish ? finish_limits(j.sd) : FinishLimits{};
     launch_raygen(j.sd, pd, b, ls);
     launches = 2;                     // with the accumulation
     const int max_paths = b.n_paths;
-    if (max_paths <= limit) {
-      launch_finish(j.sd, b, pd, 0, limit, ls);
+    if (max_paths <= limits.at_once) {
+      launch_finish(j.sd, b, pd, 0, limits.at_once, ls);
       ++launches;
     } else {
       for (int bounce = 0; bounce < j.sd.max_depth; ++bounce) {
         int q = bounce & 1;
-        if (finish && finish_check(bounce, j.sd.max_depth, max_paths, limit)) {
-          launch_finish(j.sd, b, pd, q, limit, ls);
+        if (finish && finish_check(bounce, j.sd.max_depth, max_paths, limits)) {
+          launch_finish(j.sd, b, pd, q, limits.later, ls);
           ++launches;
         }
         timed(1, [&] { launch_trace(j.sd, pd, q, 2 * max_paths, ls, trace_cap); });
@@ -1121,6 +1121,18 @@ int hasty_debug_tri_ids(hasty_job* job, int32_t* geom, int32_t* prim, size_t n) 
     as_job(job);
     if (n != job->host.tri_attr.size()) throw ApiError{HASTY_ERR_ARG, "n must equal the triangle count"};
     for (size_t i = 0; i < n; ++i) { geom[i] = int32_t(job->host.tri_attr[i].geom); prim[i] = int32_t(job->host.tri_attr[i].prim); }
+    return HASTY_OK;
+  });
+}
+
+int hasty_debug_finish_limits(hasty_job* job, int64_t* at_once, int64_t* later) {
+  return guarded([&] {
+    as_job(job);
+    if (!at_once || !later) throw ApiError{HASTY_ERR_ARG, "null argument"};
+    ck(cudaSetDevice(job->ctx->device), "cudaSetDevice");
+    const FinishLimits l = finish_limits(job->sd);
+    *at_once = l.at_once;
+    *later = l.later;
     return HASTY_OK;
   });
 }

@@ -952,7 +952,6 @@ void launch_finish_src(const Src& src, int bvh_kind, const PathsDev& p, int q, i
   const int64_t most = std::min<int64_t>(n_bound, limit);
   const int threads = most * 2 <= path_slots() ? kPathBlockThreads / 2 : kPathBlockThreads;
   const int grid = int(std::max<int64_t>(1, std::min<int64_t>(path_slots() / threads, (most + threads - 1) / threads)));
-  if (n_bound > limit) limit /= 2;
   if (bvh_kind == 1) launch_dependent(k_paths<Src, 1, true>, grid, threads, st, src, p, p, q, uint32_t(limit));
   else launch_dependent(k_paths<Src, 0, true>, grid, threads, st, src, p, p, q, uint32_t(limit));
 }
@@ -968,27 +967,48 @@ void launch_paths_packed(const ChunkTable& t, int bvh_kind, const PathsDev& slot
   launch_paths_src(t, t.n_paths, bvh_kind, slots, out, st);
 }
 
-// Batches of at most this many times the paths that the GPU holds at once
-// (78k) are finished by launch_finish from the start. Batches of n samples,
-// wavefront / finished, ms: Cornell box (tiny BVH) 64k 0.332 / 0.220, 128k
-// 0.391 / 0.350, 256k 0.517 / 0.542; textured room 256k 0.605 / 0.531, 512k
-// 0.792 / 0.929; 256k-triangle field 256k 0.636 / 0.388, 512k 0.781 / 0.655;
-// 1.02M-triangle field 256k 1.056 / 0.699, 512k 1.322 / 1.201; stress scene
-// 256k 3.410 / 2.101, 512k 4.433 / 3.608.
+// Which batches launch_finish takes, as multiples of the 78k paths that the GPU
+// holds at once. It saves a bounce's three launches, a time that grows with the
+// depth limit, and carries a path through its bounces at a half to a third of
+// the wavefront's rate, so what it may take grows with the depth too; and paths
+// lit by the sky alone are short (their light rays end at any hit, and those that
+// miss the scene end). Wavefront / finished, ms, at depths 2, 4, 8 and 12 with
+// 160k samples: textured room 0.18/0.23, 0.30/0.34, 0.50/0.42, 0.67/0.46; 52k-
+// triangle stress scene 0.30/0.38, 0.54/0.65, 0.91/0.85, 1.24/0.97; nested glass
+// 0.23/0.23, 0.44/0.47, 0.80/0.80, 1.10/0.92; fields of 15k triangles, dense,
+// 0.18/0.18, 0.30/0.23, 0.47/0.27, 0.59/0.34, of 256k 0.21/0.22, 0.34/0.28,
+// 0.48/0.30, 0.51/0.30, of 1.02M at 2, 6 and 12 0.29/0.35, 0.62/0.48, 0.93/0.54;
+// with 280k: room 0.24/0.36, 0.38/0.51, 0.59/0.59, 0.76/0.62, field of 256k
+// 0.25/0.31, 0.39/0.37, 0.56/0.41, 0.58/0.40. Cornell box (tiny BVH) at depths
+// 2, 4, 8 and 12, 78k samples 0.10/0.10, 0.17/0.15, 0.30/0.25, 0.43/0.32, 109k
+// 0.11/0.13, 0.19/0.23, 0.33/0.32, 0.46/0.37. (One limit for all depths, 3.6 and 1.7, had
+// been chosen at depths of 8 and more; at depths 2 to 6 it made such batches up
+// to 1.45 times slower.)
 constexpr double kFinishTiny = 1.7, kFinishOther = 3.6;
-int64_t finish_limit(bool tiny_bvh) { return int64_t(double(path_slots()) * (tiny_bvh ? kFinishTiny : kFinishOther)); }
+FinishLimits finish_limits(const SceneDev& sc) {
+  const double slots = double(path_slots()), depth = sc.max_depth;
+  const bool tiny = simple_trace_bvh(sc), sky_only = sc.n_light_tris == 0;
+  const double cap = tiny ? kFinishTiny : kFinishOther;
+  double f = cap;
+  if (sky_only) { if (!tiny) f = 0.75 * depth - 0.2; }
+  else f = tiny ? 0.75 + 0.095 * depth : 0.2 + 0.3 * depth;
+  FinishLimits l;
+  l.at_once = int64_t(slots * std::min(cap, std::max(tiny ? 0.9 : 1.0, f)));
+  l.later = int64_t(slots * cap / 2);
+  return l;
+}
 
-// A larger batch is offered to launch_finish (which takes half as many paths
-// of it: they have fewer bounces ahead) before every other bounce from the
+// A larger batch is offered to launch_finish (which takes FinishLimits::later
+// paths of it: they have fewer bounces ahead) before every other bounce from the
 // first at which its paths could have become few enough (scenes lose two
 // thirds of them per bounce at most), while six bounces or more are left: an
 // offer declined costs 4 us, and the last bounces of a shallow batch are
 // cheap. Stress scene at depth 32, 4.1M samples: 17.58 -> 16.79 ms; 0.6M
 // samples of the 256k-triangle field at depth 9: 0.673 -> 0.603 ms.
-bool finish_check(int bounce, int max_depth, int64_t n_paths, int64_t limit) {
+bool finish_check(int bounce, int max_depth, int64_t n_paths, const FinishLimits& l) {
   if (bounce + 6 > max_depth) return false;
   int first = 1;
-  for (int64_t n = n_paths / 3; n > limit; n /= 3) ++first;
+  for (int64_t n = n_paths / 3; n > 2 * l.later; n /= 3) ++first;
   return bounce >= first && (bounce - first) % 2 == 0;
 }
 

@@ -111,17 +111,28 @@ void PackedLanes::launch(const std::vector<PackedJob>& jobs, const std::vector<P
     launches += 1;
   } else {
     const bool finish = !(ctx->flags & HASTY_CTX_WAVEFRONT);
-    const int64_t limit = finish ? finish_limit(jobs[size_t(chunks[0].job)].simple_trace) : 0;
+    // of the chunks' limits the mean over their samples
+    FinishLimits limits;
+    if (finish) {
+      double at_once = 0.0, later = 0.0;
+      for (int c = 0; c < ct.n; ++c) {
+        const FinishLimits l = finish_limits(ct.c[c].sc);
+        const double share = double(ct.c[c].n_passes) * ct.c[c].npix / n_paths;
+        at_once += share * double(l.at_once);
+        later += share * double(l.later);
+      }
+      limits = {int64_t(at_once), int64_t(later)};
+    }
     launch_raygen_packed(ct, p, ls);
     launches += 1;
-    if (n_paths <= limit) {
-      launch_finish_packed(ct, bvh_kind, p, 0, limit, ls);
+    if (n_paths <= limits.at_once) {
+      launch_finish_packed(ct, bvh_kind, p, 0, limits.at_once, ls);
       launches += 1;
     } else {
       for (int bounce = 0; bounce < max_depth; ++bounce) {
         const int q = bounce & 1;
-        if (finish && finish_check(bounce, max_depth, n_paths, limit)) {
-          launch_finish_packed(ct, bvh_kind, p, q, limit, ls);
+        if (finish && finish_check(bounce, max_depth, n_paths, limits)) {
+          launch_finish_packed(ct, bvh_kind, p, q, limits.later, ls);
           launches += 1;
         }
         launch_trace_packed(tt, p, q, 2 * n_paths, ls, trace_cap);

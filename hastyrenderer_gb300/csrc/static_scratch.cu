@@ -112,7 +112,7 @@ extern "C" int hasty_job_render_pass_static(hasty_job* job, int pass, double* d_
     b.n_passes = 1;
     b.n_paths = npix;
     launch_raygen(job->sd, p, b, job->stream);
-    const int64_t limit = (job->ctx->flags & HASTY_CTX_WAVEFRONT) ? 0 : finish_limit(simple_trace_bvh(job->sd));
+    const int64_t limit = (job->ctx->flags & HASTY_CTX_WAVEFRONT) ? 0 : finish_limits(job->sd).at_once;
     if (job->sd.max_depth > 0 && npix <= limit) {
       launch_finish(job->sd, b, p, 0, limit, job->stream);
     } else {

@@ -213,12 +213,14 @@ void launch_paths_packed(const ChunkTable& t, int bvh_kind, const PathsDev& slot
 
 // Finishing small queues: the path kernel on a batch's own state. Carries the
 // paths of queue q (before their closest hits of this bounce) to their ends
-// if there are at most `limit` (half of it when the batch itself is larger),
-// leaving the queue empty; otherwise does nothing. Same samples, bit for bit.
-// finish_limit: the largest batch finished at bounce 0, with no other launch;
-// finish_check: whether to offer bounce `bounce` of a larger one.
-int64_t finish_limit(bool tiny_bvh);
-bool finish_check(int bounce, int max_depth, int64_t n_paths, int64_t limit);
+// if there are at most `limit`, leaving the queue empty; otherwise does nothing.
+// Same samples, bit for bit.
+// FinishLimits: the largest batch finished at bounce 0, with no other launch, and
+// the most paths of a larger one that are; finish_check: whether to offer it at
+// bounce `bounce`.
+struct FinishLimits { int64_t at_once = 0, later = 0; };
+FinishLimits finish_limits(const SceneDev& sc);
+bool finish_check(int bounce, int max_depth, int64_t n_paths, const FinishLimits& l);
 void launch_finish(const SceneDev& sc, const BatchDesc& b, const PathsDev& p, int q, int64_t limit, cudaStream_t stream);
 void launch_finish_packed(const ChunkTable& t, int bvh_kind, const PathsDev& p, int q, int64_t limit, cudaStream_t stream);
 

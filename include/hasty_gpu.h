@@ -423,6 +423,10 @@ int hasty_debug_host_trace(const char* render_job_path, int kind, const float* r
 int hasty_debug_wide_emit_check(int device, const char* render_job_path, int64_t* info, int32_t* identical);
 /* Triangle index -> (OBJ shape = Embree geomID, face = primID). */
 int hasty_debug_tri_ids(hasty_job* job, int32_t* geom, int32_t* prim, size_t n);
+/* Test hook: the most camera samples of a batch that one kernel carries from
+ * their first hits to their ends, and the most paths of a larger batch that it
+ * takes over at a later bounce. */
+int hasty_debug_finish_limits(hasty_job* job, int64_t* at_once, int64_t* later);
 /* Test hook (no device needed): the index that each 64-bit draw takes from the
  * discrete distribution with the n >= 2 cumulative values cdf[], by the
  * integer thresholds and guide table that the kernels draw with. */
