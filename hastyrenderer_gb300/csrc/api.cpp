@@ -341,16 +341,20 @@ int64_t default_capacity(int64_t npix) {
 // tracing, which is bound by instruction issue, then runs beside shading, which
 // is bound by latency, for a second set of launches and of last bounces with
 // few paths. One batch / two, ms: Cornell box (tiny BVH), depth 8, 0.26M
-// samples 0.54 / 0.64, 0.5M 0.83 / 0.72, 1M 1.44 / 1.27, 4.2M 5.03 / 4.76;
-// depth 16, 0.5M 1.14 / 1.16, 1M 1.79 / 1.70; depth 24, 2M 3.29 / 3.08.
-// 64k-triangle field, depth 10, 1M 0.73 / 0.73, 2M 1.09 / 1.06, 4.2M 1.79 /
-// 1.71; textured room, depth 8, 2.5M 2.37 / 2.27, 4.9M 4.32 / 4.18, but depth
-// 16, 4.9M 4.78 / 4.93. 1.02M-triangle field 2M 2.47 / 2.72, 5.2M 5.19 / 5.29
-// (the two lanes' tracing shares the L2); stress scene, depth 32, 2M 4.75 /
-// 5.08.
+// samples 0.54 / 0.64, 0.5M 0.83 / 0.72, 1M 1.40 / 1.26, 4.2M 5.06 / 4.78, depth
+// 2, 1M 0.60 / 0.57, 16.8M 8.78 / 8.68, depth 32, 1M 2.00 / 2.00, 4.2M 5.88 /
+// 5.63. Up to depth 9, 2.1M and 4.2M samples: textured room 1.98 / 1.96 and 3.53
+// / 3.38, 64k-triangle field 1.00 / 0.99 and 1.64 / 1.61, 128k-triangle field at
+// depth 6 1.08 / 1.06 and 1.79 / 1.73, 52k-triangle stress scene at depth 8 4.23 /
+// 4.17 and 7.91 / 7.71. At depths 10 to 12, 3.1M and 6.3M: room 2.82 / 2.93 and
+// 5.17 / 5.06, stress scene 6.51 / 6.68 and 12.15 / 11.83, 64k-triangle field 1.37
+// / 1.34 and 2.30 / 2.30. Deeper, room at 16, 4.9M 4.78 / 4.93, and of larger
+// trees, 1.02M-triangle field 2M 2.47 / 2.72, 5.2M 5.19 / 5.29 (the two lanes'
+// tracing shares the L2), stress scene at depth 32, 2M 4.75 / 5.08.
 bool worth_two_batches(const hasty_job& j, int64_t samples) {
   if (simple_trace_bvh(j.sd)) return samples >= int64_t(1) << 20;
-  return samples >= int64_t(1) << 21 && j.sd.max_depth <= 12 && j.sd.n_tris <= 1 << 17;
+  const int64_t least = int64_t(j.sd.max_depth <= 9 ? 2 : 6) << 20;
+  return samples >= least && j.sd.max_depth <= 12 && j.sd.n_tris <= 1 << 17;
 }
 
 // Passes per batch of a call: at most the paths in flight, the batches of one
