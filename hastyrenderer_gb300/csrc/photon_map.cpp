@@ -41,6 +41,8 @@ struct PmDev {
   uint32_t* start = nullptr;               // table of cell starts (PmMapDev)
   size_t start_cap = 0;
   int64_t max_table = kPmDenseCells;
+  bool any_frame = false;                  // (test hook) however few pixels the frame has
+  bool table_used = false;                 // by the last iteration's gather
   int4* cells = nullptr;
   size_t cells_cap = 0;
   int32_t* cell_count = nullptr;
@@ -445,9 +447,9 @@ void pm_iteration(hasty_job& j, PmDev& pm) {
     cells = d > kPmDenseCells ? kPmDenseCells + 1 : std::min<int64_t>(cells * d, kPmDenseCells + 1);
   }
   // The table of cell starts for 2.3 million cells takes 0.03 ms and saves the
-  // gather of 307,200 pixels 0.26 ms of 1.86 (640x480 room): worth it up to
-  // about 70 cells a pixel.
-  if (cells > 0 && cells <= std::min<int64_t>(pm.max_table, 32 * int64_t(W) * H)) {
+  // gather of 307,200 pixels 0.26 ms of 1.86 (640x480 room): it would pay up to
+  // about 70 cells a pixel there, and is made up to half of that.
+  if (cells > 0 && cells <= pm.max_table && (pm.any_frame || cells <= 32 * int64_t(W) * H)) {
     try {
       pm.start = grow(j, pm.start, pm.start_cap, size_t(cells) + 1, 0);
       map.start = pm.start;
@@ -456,6 +458,7 @@ void pm_iteration(hasty_job& j, PmDev& pm) {
     }
     if (map.start) launch_pm_starts(map, pm.start, cells, j.stream);
   }
+  pm.table_used = map.start != nullptr;
   ck(cudaGetLastError(), "photon map launch");
   ck(cudaEventRecord(ev[4], j.stream), "event");
   const float ox = halton_value(2, t), oy = halton_value(3, t);
@@ -579,6 +582,17 @@ int hasty_debug_pm_table(hasty_job* job, int64_t max_cells) {
   return guarded([&] {
     pm_job(job);
     pm_state(*job).max_table = std::min(max_cells, kPmDenseCells);
+    pm_state(*job).any_frame = true;
+    return HASTY_OK;
+  });
+}
+
+int hasty_debug_pm_table_used(hasty_job* job, int32_t* used) {
+  return guarded([&] {
+    pm_job(job);
+    if (!used) throw ApiError{HASTY_ERR_ARG, "null argument"};
+    if (!job->pm || !job->pm->initialised) throw ApiError{HASTY_ERR_ARG, "no photon-mapping iteration rendered"};
+    *used = job->pm->table_used ? 1 : 0;
     return HASTY_OK;
   });
 }

@@ -148,6 +148,7 @@ def lib() -> ctypes.CDLL:
         "hasty_pm_read_radii": [P, P, SZ, SZ],
         "hasty_pm_stats_get": [P, P],
         "hasty_debug_pm_table": [P, I64],
+        "hasty_debug_pm_table_used": [P, P],
         "hasty_debug_pm_host": [P, SZ, SZ, ctypes.c_float, P],
         "hasty_debug_pm_map": [P, P, P, P, P, P, P, P],
         "hasty_job_render_pass_static": [P, I, P],

@@ -209,8 +209,11 @@ int hasty_pm_stats_get(hasty_job* job, hasty_pm_stats* stats);
 int hasty_debug_pm_map(hasty_job* job, float* xyz, uint32_t* emission, uint32_t* index, int32_t* cells,
                        int64_t* n_photons, int64_t* n_cells, float* cell);
 /* Test hook: the gather looks cells up in a table of all cells of the map's
- * bounds only up to max_cells of them (0: always searches the cell list). */
+ * bounds only up to max_cells of them (0: always searches the cell list),
+ * however few pixels the frame has. */
 int hasty_debug_pm_table(hasty_job* job, int64_t max_cells);
+/* Test hook: whether the last iteration's gather used that table. */
+int hasty_debug_pm_table_used(hasty_job* job, int32_t* used);
 /* Test hook (no device needed): the host's part of the photon mapper's set-up
  * and of an iteration. dist: w x h distances (negative: none), replaced by the
  * footprint radii of a camera with q = tan(fov / 2); cell: the hash-cell size
