@@ -31,11 +31,11 @@ struct PmEmitOut {
 };
 
 // Photon map of one iteration: photons sorted by (cell x, y, z, emission
-// index, depth); cells sorted lexicographically with the first photon and
-// the count of each. `start` (null when the bounds hold more than
-// kPmDenseCells cells, or 32 to a pixel): for every cell of the bounds in the same order the
-// first photon not before it, and one entry past them, so the photons of
-// cells z0..z1 of a column are [start[z0], start[z1 + 1]).
+// index, depth); cells sorted lexicographically with the first photon of each.
+// `start` (null when the bounds hold more than kPmDenseCells cells, or 32 to a
+// pixel): for every cell of the bounds in the same order the first photon not
+// before it, and one entry past them, so the photons of cells z0..z1 of a column
+// are [start[z0], start[z1 + 1]).
 struct PmMapDev {
   const float4* pos;       // position, n_g . w_from
   const float4* rest;      // 2 per photon: incoming direction + emission index; flux + index in the emission
@@ -98,11 +98,11 @@ void launch_pm_place(const PhotonRec* app, uint32_t appended, const uint32_t* ba
 uint32_t pm_sort_tiles(uint32_t n);
 void launch_pm_sort_pass(const int32_t* coord, int32_t lo, int shift, uint32_t n, const uint32_t* perm_in,
                          uint32_t* perm_out, uint32_t* hist, uint32_t* scratch, cudaStream_t st);
-// Photons in sorted order (pos, rest), the cell table (x, y, z, first) with
-// counts and the cell count in device memory.
+// Photons in sorted order (pos, rest), the cell table (x, y, z, first) and the
+// number of cells in device memory.
 void launch_pm_cells(const PhotonRec* app, const uint32_t* src, const int32_t* coords, uint32_t cap, uint32_t n,
                      const uint32_t* perm, float4* pos, float4* rest, uint32_t* flag, uint32_t* cell_of, uint32_t* scratch,
-                     int4* cells, int32_t* counts, int32_t* n_cells, cudaStream_t st);
+                     int4* cells, int32_t* n_cells, cudaStream_t st);
 
 // out[0..n) = value
 void launch_pm_fill(float* out, size_t n, float value, cudaStream_t st);

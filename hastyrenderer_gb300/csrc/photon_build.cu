@@ -280,14 +280,6 @@ __global__ void __launch_bounds__(kThreads) k_cells(const int32_t* coords, uint3
   cells[cell_of[q]] = make_int4(coords[s], coords[cap + s], coords[2 * cap + s], int(q));
 }
 
-__global__ void __launch_bounds__(kThreads) k_cell_counts(const int4* cells, const int32_t* n_cells, uint32_t n,
-                                                          int32_t* counts) {
-  const int c = int(blockIdx.x * blockDim.x + threadIdx.x);
-  const int nc = *n_cells;
-  if (c >= nc) return;
-  counts[c] = (c + 1 < nc ? cells[c + 1].w : int(n)) - cells[c].w;
-}
-
 __global__ void __launch_bounds__(kThreads) k_fill(float* out, size_t n, float value) {
   const size_t i = size_t(blockIdx.x) * kThreads + threadIdx.x;
   if (i < n) out[i] = value;
@@ -362,7 +354,7 @@ void launch_pm_sort_pass(const int32_t* coord, int32_t lo, int shift, uint32_t n
 
 void launch_pm_cells(const PhotonRec* app, const uint32_t* src, const int32_t* coords, uint32_t cap, uint32_t n,
                      const uint32_t* perm, float4* pos, float4* rest, uint32_t* flag, uint32_t* cell_of, uint32_t* scratch,
-                     int4* cells, int32_t* counts, int32_t* n_cells, cudaStream_t st) {
+                     int4* cells, int32_t* n_cells, cudaStream_t st) {
   if (n == 0) {
     cudaMemsetAsync(n_cells, 0, sizeof(int32_t), st);
     return;
@@ -371,7 +363,6 @@ void launch_pm_cells(const PhotonRec* app, const uint32_t* src, const int32_t* c
   k_sorted<<<g, kThreads, 0, st>>>(app, src, coords, cap, n, perm, pos, rest, flag);
   scan_exclusive<uint32_t>(flag, n, cell_of, scratch, nullptr, reinterpret_cast<uint32_t*>(n_cells), NoVisit{}, st);
   k_cells<<<g, kThreads, 0, st>>>(coords, cap, n, perm, flag, cell_of, cells);
-  k_cell_counts<<<g, kThreads, 0, st>>>(cells, n_cells, n, counts);
 }
 
 }  // namespace hasty

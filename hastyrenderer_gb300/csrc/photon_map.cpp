@@ -45,8 +45,6 @@ struct PmDev {
   bool table_used = false;                 // by the last iteration's gather
   int4* cells = nullptr;
   size_t cells_cap = 0;
-  int32_t* cell_count = nullptr;
-  size_t counts_cap = 0;
   int32_t* n_cells = nullptr;
   // map build (photon_build.cu)
   PmStatus* status = nullptr;              // device
@@ -400,7 +398,6 @@ void pm_iteration(hasty_job& j, PmDev& pm) {
   pm.pos = grow(j, pm.pos, pm.pos_cap, cap, 0);
   pm.rest = grow(j, pm.rest, pm.rest_cap, 2 * size_t(cap), 0);
   pm.cells = grow(j, pm.cells, pm.cells_cap, cap, 0);
-  pm.cell_count = grow(j, pm.cell_count, pm.counts_cap, cap, 0);
   // coordinates: three planes of `coords_cap / 3` slots
   if (pm.coords_cap < 3 * size_t(cap)) {
     j.release(pm.coords);
@@ -430,7 +427,7 @@ void pm_iteration(hasty_job& j, PmDev& pm) {
     }
   }
   launch_pm_cells(pm.append, pm.src, pm.coords, plane, kept, perm, pm.pos, pm.rest, pm.flag, pm.cell_of, pm.scratch,
-                  pm.cells, pm.cell_count, pm.n_cells, j.stream);
+                  pm.cells, pm.n_cells, j.stream);
   ck(cudaGetLastError(), "photon map launch");
   PmMapDev map{};
   map.pos = pm.pos;
@@ -635,13 +632,12 @@ int hasty_debug_pm_map(hasty_job* job, float* xyz, uint32_t* emission, uint32_t*
     }
     if (cells && nc > 0) {
       std::vector<int4> c(static_cast<size_t>(nc));
-      std::vector<int32_t> cnt(static_cast<size_t>(nc));
       ck(cudaMemcpyAsync(c.data(), pm.cells, c.size() * sizeof(int4), cudaMemcpyDeviceToHost, job->stream), "map");
-      ck(cudaMemcpyAsync(cnt.data(), pm.cell_count, cnt.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, job->stream), "map");
       ck(cudaStreamSynchronize(job->stream), "map");
       for (size_t k = 0; k < c.size(); ++k) {
         cells[5 * k] = c[k].x; cells[5 * k + 1] = c[k].y; cells[5 * k + 2] = c[k].z;
-        cells[5 * k + 3] = c[k].w; cells[5 * k + 4] = cnt[k];
+        cells[5 * k + 3] = c[k].w;
+        cells[5 * k + 4] = (k + 1 < c.size() ? c[k + 1].w : int32_t(pm.photons)) - c[k].w;
       }
     }
     return HASTY_OK;
