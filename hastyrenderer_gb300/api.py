@@ -127,7 +127,7 @@ class RenderJob:
         check(native.lib().hasty_job_set_paths_in_flight(self._h, ctypes.c_int64(n)))
 
     def release_paths(self) -> None:
-        """Frees the path state (about 336 B per path in flight) until the next render."""
+        """Frees the path state (424 B per path in flight) until the next render."""
         check(native.lib().hasty_job_release_paths(self._h))
 
     def render_passes(self, n: int, sync: bool = False) -> None:

@@ -369,12 +369,11 @@ int passes_per_batch(const hasty_job& j, int n_passes) {
 }
 
 // Resident blocks per SM of the persistent closest-hit kernel while two
-// render lanes run: fewer than fit (9 on GB300) leaves room for the other
-// lane's shading blocks. Measured on the 1080p sphere field (M samples/s),
-// 2-pass batches: all 822, 7: 829, 6: 834, 5: 836-840, 4: 822, 3: 788;
-// 8-pass batches: all 883, 7: 897, 6: 897, 5: 900, 4: 903, 3: 865;
-// with the 256/512-thread shading blocks: all 942, 7: 938, 6: 943, 5: 948,
-// 4: 940.
+// render lanes run: fewer than fit (8 on GB300) leaves room for the other
+// lane's shading blocks. ms at 3 / 4 / 5 / 6 / 7 / all: 1080p field of 1.02M
+// triangles 30.39 / 28.31 / 28.08 / 28.24 / 28.34 / 28.17, textured room 8.22 /
+// 7.90 / 7.90 / 7.92 / 7.94 / 7.93; the stress scene and the Cornell box (whose
+// closest hits run one ray per thread) are level.
 constexpr int kLaneTraceBlocksPerSM = 5;
 }  // namespace
 

@@ -1,6 +1,8 @@
 // Photon mapper kernels: the reference's stochastic progressive photon
-// mapper (core/src/PhotonMapping.cpp) on the GPU, one thread per photon and
-// one per pixel. Compiled without FMA contraction like integrator.cu, and
+// mapper (core/src/PhotonMapping.cpp) on the GPU, in persistent kernels whose
+// lanes take the next photon or pixel when theirs has ended and go through each
+// bounce in stages with their block. Compiled without FMA contraction like
+// integrator.cu, and
 // with the same device shading routines (device_common.cuh) and traversal
 // (traverse.cuh), so each photon path and each gather path computes what the
 // CPU restatement computes for the same random stream.

@@ -117,7 +117,7 @@ __global__ void TRACE_BOUNDS(SIMPLE) k_trace(SceneDev sc, PathsDev P, int q) {
       int rid = rq[i];
       if (!HASTY_IN_BOUNDS(rid >= 0 && rid < 2 * P.capacity, BB_QUEUE)) rid = 0;
       float4 o, d;
-    ld_pair(P.ray + 2 * int64_t(rid), o, d);
+      ld_pair(P.ray + 2 * int64_t(rid), o, d);
       Hit h = trace_any<KIND>(sc.nodes, sc.isect_tris, o.x, o.y, o.z, d.x, d.y, d.z);
       P.hit[rid] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
     }
@@ -173,7 +173,7 @@ __global__ void TRACE_BOUNDS(SIMPLE) k_trace_packed(const __grid_constant__ Trac
       int rid = rq[i];
       if (!HASTY_IN_BOUNDS(rid >= 0 && rid < 2 * P.capacity, BB_QUEUE)) rid = 0;
       float4 o, d;
-    ld_pair(P.ray + 2 * int64_t(rid), o, d);
+      ld_pair(P.ray + 2 * int64_t(rid), o, d);
       const TraceChunk& c = T.c[__float_as_uint(o.w)];
       Hit h = trace_any<KIND>(c.nodes, c.tris, o.x, o.y, o.z, d.x, d.y, d.z);
       P.hit[rid] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
@@ -213,7 +213,7 @@ __global__ void TRACE_BOUNDS(false) k_trace_multi(PathsDev P, MultiDev m) {
       if (!HASTY_IN_BOUNDS(rid >= 0 && rid < 2 * P.capacity, BB_QUEUE)) rid = 0;
       const SceneDev& sc = m.jobs[m.slot_meta[rid >> 1].x].sc;
       float4 o, d;
-    ld_pair(P.ray + 2 * int64_t(rid), o, d);
+      ld_pair(P.ray + 2 * int64_t(rid), o, d);
       Hit h = trace_any<KIND>(sc.nodes, sc.isect_tris, o.x, o.y, o.z, d.x, d.y, d.z);
       P.hit[rid] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
     }
@@ -226,7 +226,7 @@ __global__ void TRACE_BOUNDS(false) k_trace_multi(PathsDev P, MultiDev m) {
         if (!HASTY_IN_BOUNDS(rid >= 0 && rid < 2 * P.capacity, BB_QUEUE)) rid = 0;
         const SceneDev& sc = m.jobs[m.slot_meta[rid >> 1].x].sc;
         float4 o, d;
-    ld_pair(P.ray + 2 * int64_t(rid), o, d);
+        ld_pair(P.ray + 2 * int64_t(rid), o, d);
         tr.init(o.x, o.y, o.z, d.x, d.y, d.z);
         tr.any = sc.n_light_tris == 0 && (rid & 1);   // as k_trace
         nodes = sc.nodes;

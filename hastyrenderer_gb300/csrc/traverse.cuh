@@ -295,7 +295,7 @@ HDI float byte_biased(uint32_t w, uint32_t k) {
 
 // (q0, q1) * a + b, each rounded once: one packed FMA on the GPU.
 HDI float2 fma2(float q0, float q1, float a, float b) {
-#if defined(__CUDA_ARCH__) && !defined(HASTY_T_NO_F2)
+#ifdef __CUDA_ARCH__
   uint64_t q, aa, bb, r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(q0), "f"(q1));
   asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));

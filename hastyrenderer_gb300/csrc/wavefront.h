@@ -1,10 +1,11 @@
 // Wavefront path state and kernel launch interface (host + device).
 //
 // One path slot per camera sample of a batch: slot = k * (W*H) + pixel for
-// pass pass_base + k. State lives in structure-of-arrays buffers in HBM;
-// each bounce runs `trace` (closest hit of every queued ray) and `shade`
-// (resolve the previous vertex's NEE and BSDF samples, shade the new vertex,
-// emit its rays). Queues are compacted with warp ballots.
+// pass pass_base + k. State lives in HBM as arrays of 32-byte records, the
+// fields that a kernel reads together; each bounce runs `trace` (closest hit of
+// every queued ray) and `shade` (resolve the previous vertex's NEE and BSDF
+// samples, shade the new vertex, emit its rays). Queues are compacted with warp
+// ballots.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -12,7 +13,7 @@
 
 namespace hasty {
 
-// flags word (stored as the w lane of PathsDev::rad)
+// flags word (w of the first half of a path's PathsDev::state record)
 enum : uint32_t {
   PF_DEPTH_MASK = 0xFFu,          // depth of the vertex the pending BRDF ray leaves from
   PF_WL_SHIFT = 8,                // wavelength + 1 (0: not chosen yet)
@@ -224,8 +225,8 @@ bool finish_check(int bounce, int max_depth, int64_t n_paths, const FinishLimits
 void launch_finish(const SceneDev& sc, const BatchDesc& b, const PathsDev& p, int q, int64_t limit, cudaStream_t stream);
 void launch_finish_packed(const ChunkTable& t, int bvh_kind, const PathsDev& p, int q, int64_t limit, cudaStream_t stream);
 
-// Closest-hit queries of arbitrary rays (n x 6 floats, device memory).
-// Rays of a caller (6 floats each) and where their closest hits go.
+// Closest hits of a caller's rays (6 floats each) and where they go, all in
+// device memory.
 struct RayLists { float* rays; int32_t* tri; float *t, *u, *v; };
 void launch_trace_rays(const SceneDev& sc, const RayLists& q, int n, cudaStream_t stream);
 
