@@ -347,13 +347,14 @@ int64_t default_capacity(int64_t npix) {
 // / 3.38, 64k-triangle field 1.00 / 0.99 and 1.64 / 1.61, 128k-triangle field at
 // depth 6 1.08 / 1.06 and 1.79 / 1.73, 52k-triangle stress scene at depth 8 4.23 /
 // 4.17 and 7.91 / 7.71. At depths 10 to 12, 3.1M and 6.3M: room 2.82 / 2.93 and
-// 5.17 / 5.06, stress scene 6.51 / 6.68 and 12.15 / 11.83, 64k-triangle field 1.37
-// / 1.34 and 2.30 / 2.30. Deeper, room at 16, 4.9M 4.78 / 4.93, and of larger
-// trees, 1.02M-triangle field 2M 2.47 / 2.72, 5.2M 5.19 / 5.29 (the two lanes'
-// tracing shares the L2), stress scene at depth 32, 2M 4.75 / 5.08.
+// 5.17 / 5.06, stress scene 6.51 / 6.68 and 12.15 / 11.83, but lit by the sky
+// alone, 64k-triangle field 1.37 / 1.34 and 2.30 / 2.30, 128k 1.49 / 1.44. Deeper,
+// room at 16, 4.9M 4.78 / 4.93, and of larger trees, 1.02M-triangle field 2M 2.47 /
+// 2.72, 5.2M 5.19 / 5.29 (the two lanes' tracing shares the L2), stress scene at
+// depth 32, 2M 4.75 / 5.08.
 bool worth_two_batches(const hasty_job& j, int64_t samples) {
   if (simple_trace_bvh(j.sd)) return samples >= int64_t(1) << 20;
-  const int64_t least = int64_t(j.sd.max_depth <= 9 ? 2 : 6) << 20;
+  const int64_t least = int64_t(j.sd.max_depth <= 9 || j.sd.n_light_tris == 0 ? 2 : 6) << 20;
   return samples >= least && j.sd.max_depth <= 12 && j.sd.n_tris <= 1 << 17;
 }
 

@@ -1,7 +1,7 @@
 """Into how many batches a call is cut, from the job's closest-hit launches (one
-per bounce and batch): two from 1M samples of a scene with a tiny BVH, from 2M of
-others up to depth 9 and 6M up to depth 12, one otherwise. The sums are those of
-single passes."""
+per bounce and batch): two from 1M samples of a scene with a tiny BVH; of others
+up to depth 12 from 2M, or from 6M where there are area lights and the depth is 10
+or more; one otherwise. The sums are those of single passes."""
 import numpy as np
 import pytest
 
@@ -11,12 +11,14 @@ SIDE = 256
 
 @pytest.mark.parametrize("kind,depth,passes,batches", [
     ("cornell", 8, 15, 1), ("cornell", 8, 16, 2), ("cornell", 30, 17, 2),
-    ("field", 9, 31, 1), ("field", 9, 32, 2), ("field", 10, 32, 1), ("field", 12, 95, 1), ("field", 12, 96, 2),
-    ("field", 13, 96, 1)])
+    ("field", 12, 31, 1), ("field", 12, 32, 2), ("field", 13, 96, 1), ("room", 9, 31, 1), ("room", 9, 32, 2),
+    ("room", 10, 32, 1), ("room", 12, 95, 1), ("room", 12, 96, 2)])
 def test_batches_of_a_call(tmp_path, kind, depth, passes, batches):
     from hastyrenderer_gb300 import RenderJob, scenes
     if kind == "cornell":
         path = scenes.cornell_box(str(tmp_path), seed=3, width=SIDE, height=SIDE, max_depth=depth)
+    elif kind == "room":
+        path = scenes.textured_room(str(tmp_path), seed=3, width=SIDE, height=SIDE, max_depth=depth, tex_size=32)
     else:
         path = scenes.sphere_field(str(tmp_path), seed=3, n_spheres=20, subdiv=2, width=SIDE, height=SIDE, max_depth=depth,
                                    env_size=(256, 128))
