@@ -975,22 +975,22 @@ void launch_paths_packed(const ChunkTable& t, int bvh_kind, const PathsDev& slot
 // miss the scene end). Wavefront / finished, ms, at depths 2, 4, 8 and 12 with
 // 160k samples: textured room 0.18/0.23, 0.30/0.34, 0.50/0.42, 0.67/0.46; 52k-
 // triangle stress scene 0.30/0.38, 0.54/0.65, 0.91/0.85, 1.24/0.97; nested glass
-// 0.23/0.23, 0.44/0.47, 0.80/0.80, 1.10/0.92; fields of 15k triangles, dense,
-// 0.18/0.18, 0.30/0.23, 0.47/0.27, 0.59/0.34, of 256k 0.21/0.22, 0.34/0.28,
-// 0.48/0.30, 0.51/0.30, of 1.02M at 2, 6 and 12 0.29/0.35, 0.62/0.48, 0.93/0.54;
-// with 280k: room 0.24/0.36, 0.38/0.51, 0.59/0.59, 0.76/0.62, field of 256k
-// 0.25/0.31, 0.39/0.37, 0.56/0.41, 0.58/0.40. Cornell box (tiny BVH) at depths
-// 2, 4, 8 and 12, 78k samples 0.10/0.10, 0.17/0.15, 0.30/0.25, 0.43/0.32, 109k
-// 0.11/0.13, 0.19/0.23, 0.33/0.32, 0.46/0.37. (One limit for all depths, 3.6 and 1.7, had
-// been chosen at depths of 8 and more; at depths 2 to 6 it made such batches up
-// to 1.45 times slower.)
+// 0.23/0.23, 0.44/0.47, 0.80/0.80, 1.10/0.92; with 280k: room 0.24/0.36, 0.38/0.51,
+// 0.59/0.59, 0.76/0.62. Sky alone, at depths 2, 3, 4 and 5 with 200k samples:
+// sparse field of 38k triangles 0.17/0.14, 0.22/0.15, 0.26/0.16, 0.28/0.16; of 512k
+// 0.25/0.31, 0.34/0.36, 0.41/0.38, 0.47/0.40; of 1.02M 0.31/0.40, 0.41/0.46,
+// 0.49/0.49, 0.57/0.52; dense, of 602 0.17/0.21, 0.23/0.26, 0.28/0.28, 0.32/0.29; all
+// gain at 6 and more. Cornell box (tiny BVH) at depths 2, 4, 8 and 12, 78k samples
+// 0.10/0.10, 0.17/0.15, 0.30/0.25, 0.43/0.32, 109k 0.11/0.13, 0.19/0.23, 0.33/0.32,
+// 0.46/0.37. (One limit for all depths, 3.6 and 1.7, had been chosen at depths of 8
+// and more; at depths 2 to 6 it made such batches up to 1.45 times slower.)
 constexpr double kFinishTiny = 1.7, kFinishOther = 3.6;
 FinishLimits finish_limits(const SceneDev& sc) {
   const double slots = double(path_slots()), depth = sc.max_depth;
   const bool tiny = simple_trace_bvh(sc), sky_only = sc.n_light_tris == 0;
   const double cap = tiny ? kFinishTiny : kFinishOther;
   double f = cap;
-  if (sky_only) { if (!tiny) f = 0.75 * depth - 0.2; }
+  if (sky_only) { if (!tiny) f = 0.85 * depth - 0.1; }
   else f = tiny ? 0.75 + 0.095 * depth : 0.2 + 0.3 * depth;
   FinishLimits l;
   l.at_once = int64_t(slots * std::min(cap, std::max(tiny ? 0.9 : 1.0, f)));
