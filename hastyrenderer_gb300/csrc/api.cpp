@@ -379,12 +379,12 @@ constexpr int kLaneTraceBlocksPerSM = 5;
 }  // namespace
 
 // Largest scene the path kernel takes by default: none. Measured on GB300
-// (M samples/s, path kernel vs wavefront): Cornell box 1024x768 475 vs 607,
-// 128x128 389 vs 496; 64k-triangle field 1024x768 924 vs 2365; 1.02M
-// triangles 256x192 318 vs 822, at 64, 96 or 128 registers per thread. Its
-// path state stays in L2, but the wavefront's shading kernels are bound by
-// load latency at 35-52% of HBM bandwidth, not by their traffic, and the
-// path kernel loses more to idle lanes, block barriers and undivided
+// (ms, path kernel / default): Cornell box 256x256, 16 passes 1.84 / 1.28;
+// 64k-triangle field 512x512, 8 passes 1.44 / 1.03; textured room 640x480, 8
+// passes 4.04 / 2.28; a 100x80 field, 4 passes, which the same kernel finishes
+// on the batch's state, 0.15 both. Its path state stays in L2, but the
+// wavefront's shading kernels are bound by load latency, not by their traffic,
+// and the path kernel loses more to idle lanes, block barriers and undivided
 // traversal than it saves. HASTY_PATH_KERNEL_TRIS (or HASTY_CTX_PATH_KERNEL)
 // selects it.
 constexpr int64_t kPathKernelMaxTris = 0;
